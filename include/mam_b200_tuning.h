@@ -14,7 +14,7 @@ extern "C" {
 
 enum mam_tune_knob {
     MAM_TUNE_FWD_VALUES = 0,   /* tile configuration of the values-only tiled forward: -1 by shape, -2 the
-                                  any-shape kernel, 0.. index mam_fwd_variant_name(0, i)                     */
+                                  any-shape kernel, 0.. index mam_fwd_variant_name(0, i): tiled, then sliced */
     MAM_TUNE_FWD_INDICES = 1,  /* the same for the index-producing forward, names from mam_fwd_variant_name(1, i) */
     MAM_TUNE_RESOLVER = 2,     /* 0 tiled index resolver (default), 1 one thread per output                   */
     MAM_TUNE_BWD_FORM = 3,     /* 0 by shape, 1 CTA-shared rows of dX, 2 separate dX and dW kernels,

@@ -14,6 +14,7 @@
 #include "mam_csr_tiled.cuh"
 #include "mam_dense_tf32.cuh"
 #include "mam_fwd_generic.cuh"
+#include "mam_fwd_sliced.cuh"
 #include "mam_fwd_tiled.cuh"
 
 using namespace mamb200;
@@ -206,15 +207,26 @@ using IdxCfg4 = FwdCfg<8, 4, 2, 4, 4, true, 1, false, true, false, true>;   // 8
 using IdxCfg5 = FwdCfg<8, 4, 2, 4, 4, true, 2, false>;          // 64x128 tile, 256 threads, A-heavy
 using IdxCfg6 = FwdCfg<4, 4, 4, 4, 4, true, 4, false>;          // 64x128 tile, 512 threads
 using IdxCfg7 = FwdCfg<4, 4, 4, 4, 4, true, 1, false, true, false, true>;   // 64x128 tile, 512 threads, paired-warp rows
-constexpr int N_VARIANTS = 8;
-const char* kValNames[N_VARIANTS] = {"val_8x8_t128x128_c256_u1_scalar", "val_8x8_t128x128_c256_u2",
+constexpr int N_TILED = 8;
+// variants N_TILED + 4 * form + log2(cluster size): the cluster-sliced kernel, forms by tile
+constexpr int N_SLICED = 12;
+constexpr int N_VARIANTS = N_TILED + N_SLICED;
+const char* kValNames[N_TILED] = {"val_8x8_t128x128_c256_u1_scalar", "val_8x8_t128x128_c256_u2",
                                      "val_8x8_t128x128_c256_u1", "val_4x8_t96x128_c384_u2", "val_4x8_t64x192_c384_u2",
                                      "val_4x8_t64x128_c256_u2_scalar", "val_4x8_t64x128_c256_u2b",
                                      "val_4x4_t128x64_c512_u4"};
-const char* kIdxNames[N_VARIANTS] = {"idx_4x8_t64x128_c256_u1_row8", "idx_4x8_t64x128_c256_u2_row8",
+const char* kIdxNames[N_TILED] = {"idx_4x8_t64x128_c256_u1_row8", "idx_4x8_t64x128_c256_u2_row8",
                                      "idx_4x8_t64x128_c256_u1", "idx_4x4_t64x128_c512_u1",
                                      "idx_8x4_t64x128_c256_u1_row8", "idx_8x4_t64x128_c256_u2",
                                      "idx_4x4_t64x128_c512_u4", "idx_4x4_t64x128_c512_u1_row8"};
+//                                 TM TN WM WN ST
+template <bool TRACK> using Sliced8 = SlicedCfg<2, 8, 1, 2, 3, TRACK>;    // 8x128 tile, 64 threads
+template <bool TRACK> using Sliced32 = SlicedCfg<4, 4, 2, 2, 3, TRACK>;   // 32x64 tile, 128 threads
+template <bool TRACK> using Sliced64 = SlicedCfg<4, 8, 4, 2, 3, TRACK>;   // 64x128 tile, 256 threads
+const char* kSlicedNames[N_SLICED] = {"sliced_t8x128_s1", "sliced_t8x128_s2", "sliced_t8x128_s4", "sliced_t8x128_s8",
+                                      "sliced_t32x64_s1", "sliced_t32x64_s2", "sliced_t32x64_s4", "sliced_t32x64_s8",
+                                      "sliced_t64x128_s1", "sliced_t64x128_s2", "sliced_t64x128_s4",
+                                      "sliced_t64x128_s8"};
 int g_variant[2] = {-1, -1};  // [with_indices]
 int g_resolve_simple = 0;      // 1: use the thread-per-output resolver (cross-check)
 
@@ -226,6 +238,59 @@ std::mutex g_static_scratch_mutex;
 int bad_ptr(const void* p) { return p == nullptr; }
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 size_t round256(size_t x) { return (x + 255) & ~size_t(255); }
+
+// K not a multiple of 4: both operands are copied once with padded rows (mam_stage_ragged_kernel) so that TMA can
+// read them, where the product is large enough for the copy's launch: at 64x257x64 (2^20 units) the any-shape kernel
+// takes about 70 us and the copy with the sliced kernel about 15.
+bool ragged_staged(int64_t M, int64_t K, int64_t N) {
+    return M > 0 && N > 0 && K > 4 && K % 4 != 0 && (double)M * (double)K * (double)N >= 1048576.0;
+}
+size_t ragged_bytes(int64_t M, int64_t K, int64_t N) {
+    const size_t pitch = (size_t)((K + 3) / 4 * 4);
+    return round256((size_t)N * pitch * 4) + round256((size_t)M * pitch * 4);
+}
+
+// The cluster-sliced forward: `slices` CTAs per tile (at most one per 32-wide chunk of K), one launch, indices
+// included.
+template <class Cfg>
+int launch_sliced(const SlicedParams& prm, int slices, const DevInfo& d, cudaStream_t st) {
+    if (Cfg::SMEM_BYTES > d.max_smem) return MAM_ERR_UNSUPPORTED;
+    CUtensorMap tmA, tmW;
+    int s = encode_rows_k(&tmA, prm.a, prm.M, prm.K, Cfg::BM);
+    if (s != MAM_OK) return s;
+    s = encode_rows_k(&tmW, prm.w, prm.N, prm.K, Cfg::BN);
+    if (s != MAM_OK) return s;
+    const long long nk = (prm.K + FWD_BK - 1) / FWD_BK;
+    while (slices > nk) slices >>= 1;
+    const long long grid = ((prm.M + Cfg::BM - 1) / Cfg::BM) * ((prm.N + Cfg::BN - 1) / Cfg::BN) * slices;
+    if (grid > 2147483647LL) return MAM_ERR_UNSUPPORTED;
+    MAM_CUDA(cudaFuncSetAttribute(mam_fwd_sliced_kernel<Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  Cfg::SMEM_BYTES));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(Cfg::THREADS);
+    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)slices;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    TimedLaunch t(MAM_KERNEL_FWD_TILED, st);
+    MAM_CUDA(cudaLaunchKernelEx(&cfg, mam_fwd_sliced_kernel<Cfg>, tmA, tmW, prm));
+    return MAM_OK;
+}
+
+template <bool TRACK>
+int run_sliced(const SlicedParams& prm, int which, const DevInfo& d, cudaStream_t st) {
+    const int slices = 1 << (which & 3);
+    switch (which >> 2) {
+        case 0: return launch_sliced<Sliced8<TRACK>>(prm, slices, d, st);
+        case 1: return launch_sliced<Sliced32<TRACK>>(prm, slices, d, st);
+        default: return launch_sliced<Sliced64<TRACK>>(prm, slices, d, st);
+    }
+}
 
 template <int R>
 int launch_csr(const float* a, const int64_t* crow, const int64_t* col, const float* val, const float* bias,
@@ -267,6 +332,63 @@ int auto_variant(bool want_idx, int64_t M, int64_t N, const DevInfo& d) {
     return variant;
 }
 
+// Predicted time of a tiled forward (with indices: and its resolver) in microseconds: `waves` rounds of tiles, each
+// nk chunks long.  With indices: 3.4 us a chunk and 42 a round give 2.95 and 3.96 ms at 12608x3072x768 and
+// 12608x768x3072 (measured 2.98 and 3.83).
+double tiled_us(int variant, bool want_idx, int64_t M, int64_t N, int64_t nk, const DevInfo& d) {
+    const long long bm = want_idx ? 64 : variant == 2 ? 128 : variant == 3 ? 96 : 64;
+    const double waves = (double)((((M + bm - 1) / bm) * ((N + 127) / 128) + d.sms - 1) / d.sms);
+    if (want_idx) return waves * (3.4 * nk + 42.0);
+    return bm == 128 ? 6.1 + 6.1 * waves * nk : bm == 96 ? 3.0 + 4.9 * waves * nk : 0.8 + waves * (3.2 * nk + 3.4);
+}
+
+// Tile configuration of a forward on matrix operands, tiled or sliced over clusters.
+//
+// The sliced kernel runs every CTA of the grid at once or nearly so; its time is a launch, the chunks of the longest
+// slice, and the outputs each CTA merges (and resolves), each with a part that grows with the CTAs per SM.  The
+// coefficients below are least-squares fits (us) to the twelve forms over seventeen shapes from 1x128x128 to
+// 3000x768x768 (K in the middle): the form so chosen is within 8 % of the best one, within 24 % at a few of the
+// smallest index-producing products.  Measured, tiled (or any-shape, below 4096 outputs) -> sliced, us:
+//            8x768x3072   64x512x512   256x512x256   777x1000x515   1024^3    1500x700x1500   1x4096x4096
+//   values   79 -> 9.1    56 -> 8.1    56 -> 8.4     105 -> 54      107->102  141 (tiled)     411 -> 31
+//   indices  105 -> 11.6  101 -> 12.7  101 -> 13.2   163 -> 77      164->147  228 (tiled)     480 -> 28
+// From four rounds of 64x128 tiles on the tiled kernels run without a comparison: their CTAs are persistent, and the
+// fits end there (12608x3072x768, eight rounds: 2.98 ms tiled, 3.13 sliced).
+int matrix_variant(bool want_idx, int64_t M, int64_t N, int64_t K, const DevInfo& d) {
+    struct Form { long long bm, bn; double fit[2][6]; };
+    static const Form forms[3] = {
+        {8, 128, {{3.05, 1.50, 0.43, 2.4, 0.0, 0.93}, {2.84, 1.19, 0.51, 20.9, 4.8, 2.26}}},
+        {32, 64, {{4.01, 1.38, 0.73, 0.5, 0.0, 0.78}, {5.86, 1.36, 0.76, 14.6, 9.6, 1.13}}},
+        {64, 128, {{5.56, 3.22, 3.49, 2.2, 0.0, 7.33}, {9.14, 3.63, 4.78, 44.3, 13.5, 16.5}}}};
+    const int64_t nk = (K + FWD_BK - 1) / FWD_BK;
+    int variant = auto_variant(want_idx, M, N, d);
+    const bool copied = K % 4 != 0;   // padded copies come first (5 us)
+    if (((M + 63) / 64) * ((N + 127) / 128) > 4LL * d.sms) return variant;
+    double best = tiled_us(variant, want_idx, M, N, nk, d) + (copied ? 5.0 : 0.0);
+    // The any-shape kernel tracks indices per k and needs no merge and no resolver: the better one where K is short
+    // and the outputs are many (4096x36x128 with indices: 13 us, sliced 32)
+    const long long gy = (M + GEN_TILE - 1) / GEN_TILE;
+    const double generic = 2.0 + 0.245 * K * (double)((gy * ((N + GEN_TILE - 1) / GEN_TILE) + d.sms - 1) / d.sms);
+    if (gy <= 65535 && generic < best) {
+        best = generic;
+        variant = -2;
+    }
+    for (int f = 0; f < 3; ++f)
+        for (int l = 0; l < 4; ++l) {
+            const long long s = 1LL << l;
+            if (s > nk) break;
+            const long long ctas = ((M + forms[f].bm - 1) / forms[f].bm) * ((N + forms[f].bn - 1) / forms[f].bn) * s;
+            const double more = (double)((ctas + d.sms - 1) / d.sms - 1), n = (double)((nk + s - 1) / s);
+            const double* c = forms[f].fit[want_idx ? 1 : 0];
+            const double us = c[0] + n * (c[1] + c[2] * more) + (c[3] + c[4] * more) / s + c[5] * more + (copied ? 5.0 : 0.0);
+            if (us < best) {
+                best = us;
+                variant = N_TILED + 4 * f + l;
+            }
+        }
+    return variant;
+}
+
 // What the im2col-mode loads can express: whole 32-channel chunks, corners and tap offsets inside the
 // instruction's fields ([-128, 127] and [0, 255] for two spatial dimensions), strides up to 8, and an
 // input of at least 128 KiB (smaller im2col maps are not encoded reliably by current drivers).
@@ -290,6 +412,10 @@ int run_tiled(const float* a, const float* w, float* y, int32_t* argmax, int32_t
     int st = MAM_OK;
     int* flag = nullptr;
     MAM_CUDA(cudaGetSymbolAddress(reinterpret_cast<void**>(&flag), g_wait_gave_up));
+    if (!cv && variant >= N_TILED) {
+        const SlicedParams sp{a, w, y, argmax, argmin, M, K, N, ep, 1.0f, flag};
+        return want_idx ? run_sliced<true>(sp, variant - N_TILED, d, cs) : run_sliced<false>(sp, variant - N_TILED, d, cs);
+    }
     FwdParams prm{y, argmax, argmin, M, K, N, ep, 1.0f, flag, Im2colRows{}, 0};
     if (cv) {
         const ConvGeom& g = cv->g;
@@ -523,12 +649,13 @@ const char* mam_fwd_variant_name(int with_indices, int variant) {
     if (variant == -1) return "auto";
     if (variant == -2) return "generic";
     if (variant < 0 || variant >= N_VARIANTS) return "";
+    if (variant >= N_TILED) return kSlicedNames[variant - N_TILED];
     return with_indices ? kIdxNames[variant] : kValNames[variant];
 }
 
 size_t mam_fwd_workspace_bytes(int64_t M, int64_t K, int64_t N, int b_layout, int want_indices) {
-    (void)M;
     (void)want_indices;
+    if ((b_layout == MAM_B_KN || b_layout == MAM_B_NK) && ragged_staged(M, K, N)) return ragged_bytes(M, K, N);
     if (b_layout == MAM_B_KN && K > 0 && N > 0 && K % 4 == 0) return round256((size_t)K * (size_t)N * 4);
     return 0;
 }
@@ -602,14 +729,12 @@ int mam_fwd_drop_f32(const float* a, const float* b, int b_layout, const float* 
 
     int variant = g_variant[want_idx ? 1 : 0];
     const bool tma_ok = (K % 4 == 0) && aligned16(a) && aligned16(b) && K / FWD_BK < 65535;
+    const bool ragged = variant == -1 && ragged_staged(M, K, N) && K / FWD_BK < 65534 && workspace != nullptr &&
+                        workspace_bytes >= ragged_bytes(M, K, N) && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0;
     if (variant == -1) {
-        if (!(tma_ok && M * N >= 4096)) {
-            variant = -2;
-        } else {
-            variant = auto_variant(want_idx, M, N, *d);
-        }
+        variant = tma_ok || ragged ? matrix_variant(want_idx, M, N, K, *d) : -2;
     }
-    if (variant >= 0 && !tma_ok) variant = -2;
+    if (variant >= 0 && !tma_ok && !ragged) variant = -2;
 
     if (variant == -2) {
         const long long gx = (N + GEN_TILE - 1) / GEN_TILE, gy = (M + GEN_TILE - 1) / GEN_TILE;
@@ -624,6 +749,18 @@ int mam_fwd_drop_f32(const float* a, const float* b, int b_layout, const float* 
         return MAM_OK;
     }
 
+    if (ragged) {
+        const int64_t pitch = (K + 3) / 4 * 4;
+        float* w = static_cast<float*>(workspace);
+        float* ac = reinterpret_cast<float*>(static_cast<char*>(workspace) + round256((size_t)N * pitch * 4));
+        const long long tiles_k = (pitch + 31) / 32, a_blocks = tiles_k * ((M + 31) / 32);
+        const long long blocks = a_blocks + tiles_k * ((N + 31) / 32);
+        if (blocks > 2147483647LL) return MAM_ERR_UNSUPPORTED;
+        mam_stage_ragged_kernel<<<(unsigned)blocks, 256, 0, cs>>>(a, b, ac, w, M, K, N, pitch, a_blocks,
+                                                                 b_layout == MAM_B_KN);
+        MAM_CUDA(cudaGetLastError());
+        return run_tiled(ac, w, y, argmax, argmin, M, pitch, N, ep, variant, *d, cs, nullptr);
+    }
     const float* w = b;
     if (b_layout == MAM_B_KN) {
         const size_t need = round256((size_t)K * (size_t)N * 4);
@@ -689,7 +826,8 @@ int mam_fwd_splits_idx_f32(const float* a, const float* w, const float* bias, co
 int mam_fwd_kn_static_f32(const float* a, const float* b, float* y, int32_t* argmax, int32_t* argmin, int64_t M,
                           int64_t K, int64_t N, void* stream) {
     if (M <= 0 || K <= 0 || N <= 0) return MAM_ERR_INVALID_ARGUMENT;
-    const size_t need = mam_fwd_workspace_bytes(M, K, N, MAM_B_KN, argmax != nullptr);
+    // (where K is not a multiple of 4 and both padded copies do not fit, the any-shape kernel runs)
+    const size_t need = K % 4 == 0 ? mam_fwd_workspace_bytes(M, K, N, MAM_B_KN, argmax != nullptr) : 0;
     if (need > MAM_STATIC_SCRATCH_BYTES || (double)K * (double)N * 4.0 > (double)MAM_STATIC_SCRATCH_BYTES)
         return MAM_ERR_STATIC_SCRATCH;
     int dev = 0;

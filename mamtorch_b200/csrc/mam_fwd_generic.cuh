@@ -172,6 +172,40 @@ mam_transpose_kernel(const float* __restrict__ in, float* __restrict__ out, long
     }
 }
 
+// Operands whose K is not a multiple of 4, copied with rows of `pitch` (K rounded up to 4) floats for the TMA kernels:
+// ac[m][k] = a[m][k], wc[n][k] = W[n][k] (or b[k][n]), the elements beyond K repeating element K-1.  A repeated
+// product can tie but never beat the original, which has the lower k, so no value and no index changes.  One launch
+// for both, 32x32 tiles, the first a_blocks blocks on a.  777 x 1001 x 515 with indices, copy included:
+// 267 us in the any-shape kernel, 4.4 + 81 us copied (sliced kernel).
+__global__ void __launch_bounds__(256)
+mam_stage_ragged_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ ac,
+                        float* __restrict__ wc, long long M, long long K, long long N, long long pitch,
+                        long long a_blocks, bool b_is_kn) {
+    __shared__ float t[32][33];
+    const long long tiles_k = (pitch + 31) / 32;
+    const bool is_a = blockIdx.x < a_blocks;
+    const long long tile = is_a ? blockIdx.x : blockIdx.x - a_blocks;
+    const long long k0 = tile % tiles_k * 32, r0 = tile / tiles_k * 32;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const long long rows = is_a ? M : N;
+    const float* src = is_a ? a : b;
+    float* dst = is_a ? ac : wc;
+    const bool transpose = !is_a && b_is_kn;
+    if (transpose) {
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const long long k = min(k0 + ty + 8 * p, K - 1), r = r0 + tx;
+            if (r < rows) t[ty + 8 * p][tx] = src[k * N + r];
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const long long k = k0 + tx, r = r0 + ty + 8 * p;
+        if (k < pitch && r < rows) dst[r * pitch + k] = transpose ? t[tx][ty + 8 * p] : src[r * K + min(k, K - 1)];
+    }
+}
+
 // out[b][c][r] = in[b][r][c] for `batch` matrices [R,C] stored back to back (blockIdx.z = b).  With R = channels
 // and C = H*W this turns an image batch [B,C,H,W] into the channels-last [B,H,W,C] the im2col-mode loads read.
 __global__ void __launch_bounds__(256)

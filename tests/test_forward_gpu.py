@@ -94,6 +94,40 @@ def test_ties_zeros_and_signs(variant, cuda):
     _check_forward(a.numpy(), np.ascontiguousarray(w.numpy().T), y_ref, imax_ref, imin_ref, cuda, variant, capi.NK)
 
 
+SLICED_SHAPES = [(1, 4, 1), (7, 260, 129), (8, 768, 300), (33, 1028, 65), (65, 36, 130), (130, 2084, 70)]
+
+
+@pytest.mark.parametrize("variant", range(8, 20))
+@pytest.mark.parametrize("shape", SLICED_SHAPES)
+def test_sliced_forms(shape, variant, cuda):
+    """Every tile and cluster size of the sliced kernel at ragged tiles, fewer chunks than slices and a ragged last
+    chunk; half of the operands are small integers, so ties cross chunks and slices.  Bit for bit, the oracle's."""
+    M, K, N = shape
+    g = torch.Generator().manual_seed(M * 5 + K * 11 + N)
+    a = torch.randn(M, K, generator=g)
+    w = torch.randn(N, K, generator=g) * K ** -0.5
+    a[: M // 2] = torch.randint(-2, 3, (M // 2, K), generator=g).float()
+    w[: N // 2] = torch.randint(-2, 3, (N // 2, K), generator=g).float()
+    y_ref, imax_ref, imin_ref = c_oracle.forward(a.numpy(), w.numpy(), b_is_nk=True)
+    _check_forward(a.numpy(), np.ascontiguousarray(w.numpy().T), y_ref, imax_ref, imin_ref, cuda, variant, capi.NK)
+
+
+@pytest.mark.parametrize("layout", [capi.KN, capi.NK])
+@pytest.mark.parametrize("shape", [(64, 257, 64), (131, 1001, 129), (1, 2047, 600), (700, 33, 515), (2100, 70, 1030)])
+def test_ragged_k(shape, layout, cuda):
+    """K that is no multiple of 4, large enough for the padded copies: the automatic choice against the oracle, with
+    ties at the last (repeated) element."""
+    M, K, N = shape
+    g = torch.Generator().manual_seed(M + K * 3 + N)
+    a = torch.randn(M, K, generator=g)
+    w = torch.randn(N, K, generator=g) * K ** -0.5
+    a[::2], w[::2] = a[::2].round(), w[::2].round()
+    a[0, -1], w[0, -1], w[-1, -1] = 40.0, 40.0, -40.0
+    y_ref, imax_ref, imin_ref = c_oracle.forward(a.numpy(), w.numpy(), b_is_nk=True)
+    assert imax_ref[0, 0] == K - 1
+    _check_forward(a.numpy(), np.ascontiguousarray(w.numpy().T), y_ref, imax_ref, imin_ref, cuda, -1, layout)
+
+
 RESOLVER_SHAPES = [(300, 260, 200), (65, 4, 63), (129, 2080, 131), (257, 96, 129), (520, 2500, 140), (64, 2048, 64),
                    (1, 64, 1), (200, 416, 136)]
 
