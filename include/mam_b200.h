@@ -351,6 +351,12 @@ int mam_spmm_csr_ws_f32(const int64_t* crow, const int64_t* col, const float* va
  * (mamtorch/nn/v4/fullyconnected.py:141, mamtorch/kernel/v4/csrc/cuda/fullyconnected.cu:66). */
 int mam_transpose_f32(const float* in, float* out, int64_t R, int64_t C, void* stream);
 
+/* out[n] = sum over m of in[m][n], in fp32 [M,N] row-major; the sums' order is fixed.  The workspace holds the
+ * partial sums of row slabs (4-byte aligned). */
+size_t mam_colsum_workspace_bytes(int64_t M, int64_t N);
+int mam_colsum_f32(const float* in, float* out, int64_t M, int64_t N, void* workspace, size_t workspace_bytes,
+                   void* stream);
+
 #ifdef __cplusplus
 }
 #endif

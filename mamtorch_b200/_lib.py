@@ -58,6 +58,8 @@ ABI = {
     "mam_spmm_csr_f32": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "mam_spmm_csr_workspace_bytes": (ctypes.c_size_t, [_i64, _i64, _i64, _i64]),
     "mam_spmm_csr_ws_f32": (_i32, [_vp, _vp, _vp, _i64, _vp, _vp, _i64, _i64, _i64, _vp, ctypes.c_size_t, _vp]),
+    "mam_colsum_workspace_bytes": (_sz, [_i64, _i64]),
+    "mam_colsum_f32": (_i32, [_vp, _vp, _i64, _i64, _vp, _sz, _vp]),
     "mam_transpose_f32": (_i32, [_vp, _vp, _i64, _i64, _vp]),
 }
 

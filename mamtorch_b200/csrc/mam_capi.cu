@@ -9,6 +9,7 @@
 #include "../../include/mam_b200.h"
 #include "../../include/mam_b200_tuning.h"
 #include "mam_bwd.cuh"
+#include "mam_colsum.cuh"
 #include "mam_conv.cuh"
 #include "mam_csr.cuh"
 #include "mam_csr_tiled.cuh"
@@ -658,6 +659,35 @@ size_t mam_fwd_workspace_bytes(int64_t M, int64_t K, int64_t N, int b_layout, in
     if ((b_layout == MAM_B_KN || b_layout == MAM_B_NK) && ragged_staged(M, K, N)) return ragged_bytes(M, K, N);
     if (b_layout == MAM_B_KN && K > 0 && N > 0 && K % 4 == 0) return round256((size_t)K * (size_t)N * 4);
     return 0;
+}
+
+// Slabs of rows for mam_colsum_f32: about four CTAs per SM and at least 64 rows each.
+static int64_t colsum_slabs(int64_t M, int64_t N) {
+    const int64_t groups = (N + COLSUM_COLS - 1) / COLSUM_COLS;
+    int64_t slabs = (8 * 148 + groups - 1) / groups;
+    if (slabs > (M + 63) / 64) slabs = (M + 63) / 64;
+    return slabs < 1 ? 1 : slabs;
+}
+
+size_t mam_colsum_workspace_bytes(int64_t M, int64_t N) {
+    if (M <= 0 || N <= 0) return 0;
+    return (size_t)colsum_slabs(M, N) * (size_t)N * 4;
+}
+
+int mam_colsum_f32(const float* in, float* out, int64_t M, int64_t N, void* workspace, size_t workspace_bytes,
+                   void* stream) {
+    if (bad_ptr(in) || bad_ptr(out) || M <= 0 || N <= 0) return MAM_ERR_INVALID_ARGUMENT;
+    const int64_t slabs = colsum_slabs(M, N), groups = (N + COLSUM_COLS - 1) / COLSUM_COLS;
+    if (groups > 2147483647LL) return MAM_ERR_UNSUPPORTED;
+    if (workspace == nullptr || workspace_bytes < mam_colsum_workspace_bytes(M, N)) return MAM_ERR_WORKSPACE;
+    const int threads = COLSUM_COLS * COLSUM_LANES;
+    float* part = static_cast<float*>(workspace);
+    mam_colsum_kernel<<<dim3((unsigned)groups, (unsigned)slabs), threads, 0, (cudaStream_t)stream>>>(
+        in, part, M, N, (M + slabs - 1) / slabs);
+    MAM_CUDA(cudaGetLastError());
+    mam_colsum_kernel<<<dim3((unsigned)groups), threads, 0, (cudaStream_t)stream>>>(part, out, slabs, N, slabs);
+    MAM_CUDA(cudaGetLastError());
+    return MAM_OK;
 }
 
 int mam_transpose_f32(const float* in, float* out, int64_t R, int64_t C, void* stream) {

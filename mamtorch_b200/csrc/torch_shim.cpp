@@ -434,6 +434,21 @@ at::Tensor conv_channels_last(const at::Tensor& x) {
 }
 // A fresh contiguous [C,R] transpose of the matrix a[R,C] (the same batched-transpose kernel, one image of R
 // channels and C pixels); several times faster than a strided torch copy.
+at::Tensor column_sum(const at::Tensor& a) {
+    TORCH_CHECK(a.is_cuda() && a.scalar_type() == at::kFloat && a.dim() == 2, "a must be a float32 CUDA matrix");
+    auto ac = a.contiguous();
+    const int64_t M = ac.size(0), N = ac.size(1);
+    c10::cuda::CUDAGuard guard(a.device());
+    if (M == 0 || N == 0) return at::zeros({N}, ac.options());
+    auto out = at::empty({N}, ac.options());
+    const size_t ws_bytes = mam_colsum_workspace_bytes(M, N);
+    auto ws = at::empty({(int64_t)ws_bytes}, ac.options().dtype(at::kByte));
+    auto stream = at::cuda::getCurrentCUDAStream();
+    check_status(mam_colsum_f32(ac.data_ptr<float>(), out.data_ptr<float>(), M, N, ws.data_ptr(), ws_bytes,
+                                stream.stream()),
+                 "mam_colsum_f32");
+    return out;
+}
 at::Tensor transpose2d(const at::Tensor& a) {
     TORCH_CHECK(a.is_cuda() && a.scalar_type() == at::kFloat && a.dim() == 2, "a must be a float32 CUDA matrix");
     auto ac = a.contiguous();
@@ -838,6 +853,7 @@ TORCH_LIBRARY(mamtorch_b200, m) {
     m.def("linear_backward_splits(Tensor x, Tensor weight, Tensor grad, Tensor argmax, Tensor argmin, float scale) -> Tensor[]");
     m.def("conv_channels_last(Tensor x) -> Tensor");
     m.def("transpose2d(Tensor a) -> Tensor");
+    m.def("column_sum(Tensor a) -> Tensor");
     m.def("conv_forward_implicit(Tensor x_nhwc, Tensor w_taps, Tensor? bias, Tensor? dense, float alpha, float beta, int kH, int kW, int sh, int sw, int ph, int pw, bool need_indices) -> Tensor[]");
     m.def("conv_implicit_applies(int B, int C, int H, int W, int kH, int kW, int sh, int sw, int ph, int pw) -> bool", &conv_implicit_applies);
     m.def("conv_col2im(Tensor cols_t, int B, int C, int H, int W, int kH, int kW, int sh, int sw, int ph, int pw) -> Tensor");
@@ -865,6 +881,7 @@ TORCH_LIBRARY_IMPL(mamtorch_b200, CUDA, m) {
     m.impl("conv_forward_implicit", &conv_forward_implicit);
     m.impl("conv_channels_last", &conv_channels_last);
     m.impl("transpose2d", &transpose2d);
+    m.impl("column_sum", &column_sum);
     m.impl("linear_forward_splits", &linear_forward_splits);
     m.impl("linear_forward_splits_idx", &linear_forward_splits_idx);
     m.impl("linear_backward_splits", &linear_backward_splits);

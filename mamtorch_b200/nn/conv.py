@@ -109,7 +109,7 @@ class _MamConv2d(torch.autograd.Function):
                     dx = _ops.conv_col2im(cols_t, B, C, H, W, kH, kW, sh, sw, ph, pw)
             dw = dw2d.view(Fo, C, kH, kW)
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            dbias = g2d.sum(0)
+            dbias = MF.bias_grad(g2d)
         if ctx.has_dense and ctx.needs_input_grad[3]:
             ddense = gy * ctx.beta
         return dx, dw, dbias, ddense, None, None, None, None, None

@@ -22,6 +22,7 @@ import math
 import torch
 from torch import Tensor, nn
 
+from ..nn import functional as MF
 from .kernel.v1 import mam_linear_csr
 
 __all__ = ["magnitude_threshold", "global_magnitude_threshold", "magnitude_keep_mask", "PrunedFullyConnected"]
@@ -82,7 +83,7 @@ class _MamLinearCsrKept(torch.autograd.Function):
         x, w, argmax, argmin = ctx.saved_tensors
         gy = gy.contiguous()
         dx, dw = torch.ops.mamtorch_b200.linear_backward(x, w, gy, argmax, argmin, 1.0)
-        dbias = gy.sum(0) if ctx.has_bias and ctx.needs_input_grad[5] else None
+        dbias = MF.bias_grad(gy) if ctx.has_bias and ctx.needs_input_grad[5] else None
         return dx, None, None, None, dw, dbias, None, None
 
 

@@ -161,3 +161,14 @@ def test_selection_count_large(cuda):
     hmax, hmin = capi.selcount(imax.to(cuda), imin.to(cuda), K)
     rmax, rmin = mam_oracle.selection_hits(imax, imin, K)
     assert torch.equal(hmax.cpu(), rmax) and torch.equal(hmin.cpu(), rmin)
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (63, 31), (64, 33), (4097, 32), (129, 4099), (70001, 17), (12608, 768)])
+def test_column_sum(shape, cuda):
+    """Column sums against float64 at the edges of slabs, lanes and column groups.  Each sum is a tree of at most
+    M/64 + 64 sequential fp32 additions, so its error stays below (M/64 + 64) * 2^-24 of the sum of magnitudes."""
+    M, N = shape
+    a = torch.randn(M, N, generator=torch.Generator().manual_seed(M + N)).to(cuda)
+    got = torch.ops.mamtorch_b200.column_sum(a).double()
+    bound = (M / 64 + 64) * 2.0 ** -24 * a.double().abs().sum(0)
+    assert got.shape == (N,) and bool(((got - a.double().sum(0)).abs() <= bound).all())
