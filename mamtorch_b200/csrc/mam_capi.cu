@@ -763,6 +763,14 @@ int mam_fwd_drop_f32(const float* a, const float* b, int b_layout, const float* 
                         workspace_bytes >= ragged_bytes(M, K, N) && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0;
     if (variant == -1) {
         variant = tma_ok || ragged ? matrix_variant(want_idx, M, N, K, *d) : -2;
+        // b[K,N] without scratch for its copy: served by the any-shape kernel below 4096 outputs, refused above,
+        // whichever kernel the sizes would take with it
+        if (tma_ok && b_layout == MAM_B_KN &&
+            (workspace == nullptr || workspace_bytes < round256((size_t)K * (size_t)N * 4) ||
+             (reinterpret_cast<uintptr_t>(workspace) & 255u))) {
+            if (M * N >= 4096) return MAM_ERR_WORKSPACE;
+            variant = -2;
+        }
     }
     if (variant >= 0 && !tma_ok && !ragged) variant = -2;
 

@@ -128,6 +128,26 @@ def test_ragged_k(shape, layout, cuda):
     _check_forward(a.numpy(), np.ascontiguousarray(w.numpy().T), y_ref, imax_ref, imin_ref, cuda, -1, layout)
 
 
+@pytest.mark.parametrize("shape,status", [((8, 64, 100), 0), ((1, 1024, 4095), 0), ((64, 36, 64), 3), ((131, 1001, 129), 0)])
+def test_column_major_weight_without_workspace(shape, status, cuda):
+    """b[K,N] and no scratch: small products and K % 4 != 0 run in the any-shape kernel, others are refused."""
+    from mamtorch_b200 import _lib
+
+    M, K, N = shape
+    g = torch.Generator().manual_seed(M + K + N)
+    a, b = torch.randn(M, K, generator=g).to(cuda), torch.randn(K, N, generator=g).to(cuda)
+    y = torch.empty(M, N, device=cuda)
+    imax, imin = torch.empty_like(y, dtype=torch.int32), torch.empty_like(y, dtype=torch.int32)
+    st = _lib.lib().mam_fwd_f32(capi._ptr(a), capi._ptr(b), capi.KN, None, None, 0, 1.0, 0.0, capi._ptr(y),
+                                capi._ptr(imax), capi._ptr(imin), M, K, N, None, 0, capi._stream())
+    assert st == status
+    if status == 0:
+        y_ref, imax_ref, imin_ref = c_oracle.forward(a.cpu().numpy(), np.ascontiguousarray(b.cpu().numpy().T), b_is_nk=True)
+        assert torch.equal(y.cpu(), torch.from_numpy(y_ref))
+        assert torch.equal(imax.cpu().long(), torch.from_numpy(imax_ref))
+        assert torch.equal(imin.cpu().long(), torch.from_numpy(imin_ref))
+
+
 RESOLVER_SHAPES = [(300, 260, 200), (65, 4, 63), (129, 2080, 131), (257, 96, 129), (520, 2500, 140), (64, 2048, 64),
                    (1, 64, 1), (200, 416, 136)]
 
