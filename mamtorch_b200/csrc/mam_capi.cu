@@ -759,7 +759,7 @@ int mam_fwd_drop_f32(const float* a, const float* b, int b_layout, const float* 
 
     int variant = g_variant[want_idx ? 1 : 0];
     const bool tma_ok = (K % 4 == 0) && aligned16(a) && aligned16(b) && K / FWD_BK < 65535;
-    const bool ragged = variant == -1 && ragged_staged(M, K, N) && K / FWD_BK < 65534 && workspace != nullptr &&
+    const bool ragged = variant != -2 && ragged_staged(M, K, N) && K / FWD_BK < 65534 && workspace != nullptr &&
                         workspace_bytes >= ragged_bytes(M, K, N) && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0;
     if (variant == -1) {
         variant = tma_ok || ragged ? matrix_variant(want_idx, M, N, K, *d) : -2;

@@ -285,8 +285,10 @@ mam_fwd_sliced_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             const int imax = first_in_chunk(prm.a, prm.w, m, nq, M, N, K, chi, hi, lane);
             const int imin = first_in_chunk(prm.a, prm.w, m, nq, M, N, K, clo, lo, lane);
             if (mine) {
-                prm.argmax[m * N + n] = imax;
-                prm.argmin[m * N + n] = imin;
+                // an extreme that never left its start (products all NaN or on the wrong infinity) keeps k = 0, as
+                // strict compares leave it (the any-shape kernel)
+                prm.argmax[m * N + n] = hi > -INFINITY ? imax : 0;
+                prm.argmin[m * N + n] = lo < INFINITY ? imin : 0;
             }
         }
     }

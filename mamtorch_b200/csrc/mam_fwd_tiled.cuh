@@ -743,7 +743,10 @@ mam_resolve_tiled_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
                 const int gq = (r + lane) & 7;
                 if (qm[r] == best) bq = min(bq, gq);
             }
-            bq = min(bq, nq - 1);  // only reachable when every product is NaN
+            // no product above -inf (all of them NaN or -inf): the chunk's first k, as strict compares from -inf
+            // leave it (the any-shape kernel); a group beyond nq holds no k of the row and must not be named
+            const bool none = !(best > -INFINITY);
+            if (none) bq = 0;
             // first element of group bq equal to the extreme
             const ulonglong2 av = lds128_s(ap + ((uint32_t)bq << 4));
             const ulonglong2 wv = lds128_s(wp + ((uint32_t)bq << 4));
@@ -753,7 +756,7 @@ mam_resolve_tiled_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             int e = 3;
             if (p2 == best) e = 2;
             if (p1 == best) e = 1;
-            if (p0 == best) e = 0;
+            if (none || p0 == best) e = 0;
             // k_offset: the problem is a slice of a wider K (slices of the module's `splits`); indices leave
             // in the numbering of the whole row
             const int kbest = CONV ? kout0 + (bq * 4 + e) * kout_step : kout0 + bq * 4 + e + k_offset;

@@ -391,3 +391,17 @@ def test_no_patch_rows_for_channel_counts_that_are_not_multiples_of_32(geom, rel
         yr.backward(gy)
         assert_grad_close(xd.grad.cpu().numpy(), xr.grad.cpu().numpy())
         assert_grad_close(wd.grad.cpu().numpy(), wr.grad.cpu().numpy())
+
+
+@pytest.mark.parametrize("order", ["unfold", "taps"])
+@pytest.mark.parametrize("channels", [3, 32, 33])
+def test_patches_of_nan_select_index_zero(channels, order, cuda):
+    """An image of NaN (a diverged step) gives every one of its outputs index 0, never one outside the weight."""
+    from mamtorch_b200.nn.conv import mam_conv2d
+
+    g = torch.Generator().manual_seed(channels)
+    x, w = torch.randn(4, channels, 32, 33, generator=g), torch.randn(40, channels, 3, 3, generator=g)
+    x[1] = float("nan")
+    _, imax, imin = mam_conv2d(x.to(cuda), w.to(cuda), None, 1, 0, reduction_order=order)
+    for idx in (imax, imin):
+        assert int(idx.min()) >= 0 and int(idx.max()) < channels * 9 and not bool(idx[1].any())

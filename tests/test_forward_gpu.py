@@ -128,6 +128,36 @@ def test_ragged_k(shape, layout, cuda):
     _check_forward(a.numpy(), np.ascontiguousarray(w.numpy().T), y_ref, imax_ref, imin_ref, cuda, -1, layout)
 
 
+@pytest.mark.parametrize("layout", [capi.KN, capi.NK])
+@pytest.mark.parametrize("variant", [-2, -1, 0, 2, 8, 13, 19])   # any-shape, by size, tiled + resolver, sliced
+@pytest.mark.parametrize("shape", [(1500, 5, 150), (900, 9, 140), (38000, 9, 100), (400, 25, 131), (300, 27, 130),
+                                   (300, 33, 130), (260, 36, 130), (131, 100, 129), (50, 36, 60)])
+def test_nan_and_infinite_products(shape, variant, layout, cuda):
+    """Rows and weights of NaN and infinities on every route: indices inside [0, K) and the oracle's, 0 where no
+    product is above -inf (max) or below +inf (min)."""
+    M, K, N = shape
+    nan, inf = float("nan"), float("inf")
+    g = torch.Generator().manual_seed(M + K + N)
+    a, w = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g)
+    a[0], a[1], a[2], a[3] = nan, inf, -inf, 0.0
+    a[4, : K // 2], a[4, K // 2:] = nan, -inf
+    a[5, : K // 2], a[5, K // 2:] = nan, inf
+    a[6, K - 1], a[-1] = inf, nan
+    w[0], w[1], w[2], w[3], w[4, 0], w[-1] = w[0].abs(), -w[1].abs(), 0.0, nan, -inf, nan
+    y_ref, imax_ref, imin_ref = c_oracle.forward(a.numpy(), w.numpy(), b_is_nk=True)
+    assert (imax_ref[0] == 0).all() and (imin_ref[:, 3] == 0).all()
+    b = (w.T.contiguous() if layout == capi.KN else w).to(cuda)
+    capi.set_variant(True, variant)
+    try:
+        y, imax, imin = capi.forward(a.to(cuda), b, layout)
+    finally:
+        capi.set_variant(True, -1)
+    assert capi.device_flag_ok()
+    assert torch.equal(imax.cpu().long(), torch.from_numpy(imax_ref))
+    assert torch.equal(imin.cpu().long(), torch.from_numpy(imin_ref))
+    assert np.array_equal(y.cpu().numpy(), y_ref, equal_nan=True)
+
+
 @pytest.mark.parametrize("shape,status", [((8, 64, 100), 0), ((1, 1024, 4095), 0), ((64, 36, 64), 3), ((131, 1001, 129), 0)])
 def test_column_major_weight_without_workspace(shape, status, cuda):
     """b[K,N] and no scratch: small products and K % 4 != 0 run in the any-shape kernel, others are refused."""
