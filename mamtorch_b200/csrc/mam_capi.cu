@@ -56,6 +56,15 @@ int device_info(const DevInfo** out) {
     return d.major == 10 ? MAM_OK : MAM_ERR_NOT_SM100;
 }
 
+// What the size queries plan with: the current device, or a B200's 148 SMs where there is none (they need no GPU).
+DevInfo plan_dev() {
+    const DevInfo* d = nullptr;
+    if (device_info(&d) == MAM_OK) return *d;
+    DevInfo b200;
+    b200.sms = 148;
+    return b200;
+}
+
 // ---- optional per-kernel event timing (mam_timer_arm) ----
 struct KernelTimer {
     void** starts = nullptr;
@@ -333,14 +342,25 @@ int auto_variant(bool want_idx, int64_t M, int64_t N, const DevInfo& d) {
     return variant;
 }
 
-// Predicted time of a tiled forward (with indices: and its resolver) in microseconds: `waves` rounds of tiles, each
-// nk chunks long.  With indices: 3.4 us a chunk and 42 a round give 2.95 and 3.96 ms at 12608x3072x768 and
-// 12608x768x3072 (measured 2.98 and 3.83).
-double tiled_us(int variant, bool want_idx, int64_t M, int64_t N, int64_t nk, const DevInfo& d) {
-    const long long bm = want_idx ? 64 : variant == 2 ? 128 : variant == 3 ? 96 : 64;
-    const double waves = (double)((((M + bm - 1) / bm) * ((N + 127) / 128) + d.sms - 1) / d.sms);
-    if (want_idx) return waves * (3.4 * nk + 42.0);
-    return bm == 128 ? 6.1 + 6.1 * waves * nk : bm == 96 ? 3.0 + 4.9 * waves * nk : 0.8 + waves * (3.2 * nk + 3.4);
+// The two padded copies of a product whose K is no multiple of 4: a launch, the bytes and the 32x32 tiles (us; fit to 98
+// products whose copies took 2 to 610 us, within 40 %).
+double copies_us(int64_t M, int64_t K, int64_t N) {
+    const double pitch = (double)((K + 3) / 4 * 4), tiles_k = (double)((K + 31) / 32);
+    return 2.0 + ((double)M + (double)N) * pitch * 8e-7 + (double)((M + 31) / 32 + (N + 31) / 32) * tiles_k * 1.6e-3;
+}
+
+// Predicted time (us) of a tiled forward.  With indices the resolver is included, whose rounds cost by the share of their
+// 128 columns that exist: least-squares fit to 67 products of 64 to 400000 rows, 6 to 930 k and 1 to 4019 columns, within
+// 35 % (15470x144x65, two rounds: 80, measured 76).  Values: up to four rounds by whole chunks; beyond, where K may be
+// short (the any-shape kernel is only compared with then), by K: fit to 83 such products within 33 %.
+double tiled_us(int variant, bool want_idx, int64_t M, int64_t N, int64_t K, bool many, const DevInfo& d) {
+    const long long bm = want_idx ? 64 : variant == 2 ? 128 : variant == 3 ? 96 : 64, ntn = (N + 127) / 128;
+    const double rounds = (double)(((M + bm - 1) / bm * ntn + d.sms - 1) / d.sms), nk = (double)((K + FWD_BK - 1) / FWD_BK);
+    if (want_idx) return 5.0 + rounds * (0.096 * K + 0.69 * nk + 5.9 + 28.4 * (double)N / (128.0 * ntn));
+    if (!many) return bm == 128 ? 6.1 + 6.1 * rounds * nk : bm == 96 ? 3.0 + 4.9 * rounds * nk : 0.8 + rounds * (3.2 * nk + 3.4);
+    return bm == 128 ? 1.0 + rounds * (0.166 * K + 0.75 * nk + 6.7)
+         : bm == 96  ? 1.4 + rounds * (0.135 * K + 0.36 * nk + 3.7)
+                     : 1.5 + rounds * (0.089 * K + 0.31 * nk + 3.4);
 }
 
 // Tile configuration of a forward on matrix operands, tiled or sliced over clusters.
@@ -353,9 +373,14 @@ double tiled_us(int variant, bool want_idx, int64_t M, int64_t N, int64_t nk, co
 //            8x768x3072   64x512x512   256x512x256   777x1000x515   1024^3    1500x700x1500   1x4096x4096
 //   values   79 -> 9.1    56 -> 8.1    56 -> 8.4     105 -> 54      107->102  141 (tiled)     411 -> 31
 //   indices  105 -> 11.6  101 -> 12.7  101 -> 13.2   163 -> 77      164->147  228 (tiled)     480 -> 28
-// From four rounds of 64x128 tiles on the tiled kernels run without a comparison: their CTAs are persistent, and the
-// fits end there (12608x3072x768, eight rounds: 2.98 ms tiled, 3.13 sliced).
-int matrix_variant(bool want_idx, int64_t M, int64_t N, int64_t K, const DevInfo& d) {
+// Beyond four rounds of 64x128 tiles the sliced forms are not considered: the tiled kernels' CTAs are persistent, and
+// the fits end there (12608x3072x768, eight rounds: 2.98 ms tiled, 3.13 sliced).  With K a multiple of 4 the tiled
+// kernels run there without a comparison.  Otherwise the any-shape kernel is the other choice.  Any-shape :
+// copies + tiled + resolver, measured, us:
+//            65536x27x64   401408x5x64  401408x147x64  401408x147x128  12608x77x768  8192x131x4096  12608x769x3072
+//   indices  52 : 229      115 : 1153   1529 : 1709    2987 : 2239     305 : 342     1715 : 1340    11109 : 3885
+//   values   52 : 58       108 : 240    1517 : 948     2970 : 944      295 : 103     1711 : 474     11108 : 2615
+int matrix_variant(bool want_idx, int64_t M, int64_t N, int64_t K, int b_layout, const DevInfo& d) {
     struct Form { long long bm, bn; double fit[2][6]; };
     static const Form forms[3] = {
         {8, 128, {{3.05, 1.50, 0.43, 2.4, 0.0, 0.93}, {2.84, 1.19, 0.51, 20.9, 4.8, 2.26}}},
@@ -363,14 +388,23 @@ int matrix_variant(bool want_idx, int64_t M, int64_t N, int64_t K, const DevInfo
         {64, 128, {{5.56, 3.22, 3.49, 2.2, 0.0, 7.33}, {9.14, 3.63, 4.78, 44.3, 13.5, 16.5}}}};
     const int64_t nk = (K + FWD_BK - 1) / FWD_BK;
     int variant = auto_variant(want_idx, M, N, d);
-    const bool copied = K % 4 != 0;   // padded copies come first (5 us)
-    if (((M + 63) / 64) * ((N + 127) / 128) > 4LL * d.sms) return variant;
-    double best = tiled_us(variant, want_idx, M, N, nk, d) + (copied ? 5.0 : 0.0);
+    const bool copied = K % 4 != 0;
+    // what the TMA kernels need first and the any-shape kernel does not: padded copies, or b[K,N] transposed
+    const double copies = copied ? copies_us(M, K, N) : b_layout == MAM_B_KN ? 1.0 + (double)K * (double)N * 1.5e-6 : 0.0;
+    const bool many = ((M + 63) / 64) * ((N + 127) / 128) > 4LL * d.sms;
+    double best = tiled_us(variant, want_idx, M, N, K, many, d) + copies;
+    const long long gy = (M + GEN_TILE - 1) / GEN_TILE;
+    const double rounds = (double)((gy * ((N + GEN_TILE - 1) / GEN_TILE) + d.sms - 1) / d.sms);
+    const bool fits = gy <= 65535;   // the any-shape kernel's grid
+    if (many) {
+        // (5 % for it: it needs no scratch; 150 products, fit within 17 %)
+        const bool any_shape = copied && fits && 1.5 + rounds * (0.23 * K + 0.96) < 1.05 * best;
+        return any_shape ? -2 : variant;
+    }
     // The any-shape kernel tracks indices per k and needs no merge and no resolver: the better one where K is short
     // and the outputs are many (4096x36x128 with indices: 13 us, sliced 32)
-    const long long gy = (M + GEN_TILE - 1) / GEN_TILE;
-    const double generic = 2.0 + 0.245 * K * (double)((gy * ((N + GEN_TILE - 1) / GEN_TILE) + d.sms - 1) / d.sms);
-    if (gy <= 65535 && generic < best) {
+    const double generic = 2.0 + 0.245 * K * rounds;
+    if (fits && generic < best) {
         best = generic;
         variant = -2;
     }
@@ -381,7 +415,7 @@ int matrix_variant(bool want_idx, int64_t M, int64_t N, int64_t K, const DevInfo
             const long long ctas = ((M + forms[f].bm - 1) / forms[f].bm) * ((N + forms[f].bn - 1) / forms[f].bn) * s;
             const double more = (double)((ctas + d.sms - 1) / d.sms - 1), n = (double)((nk + s - 1) / s);
             const double* c = forms[f].fit[want_idx ? 1 : 0];
-            const double us = c[0] + n * (c[1] + c[2] * more) + (c[3] + c[4] * more) / s + c[5] * more + (copied ? 5.0 : 0.0);
+            const double us = c[0] + n * (c[1] + c[2] * more) + (c[3] + c[4] * more) / s + c[5] * more + copies;
             if (us < best) {
                 best = us;
                 variant = N_TILED + 4 * f + l;
@@ -655,8 +689,12 @@ const char* mam_fwd_variant_name(int with_indices, int variant) {
 }
 
 size_t mam_fwd_workspace_bytes(int64_t M, int64_t K, int64_t N, int b_layout, int want_indices) {
-    (void)want_indices;
-    if ((b_layout == MAM_B_KN || b_layout == MAM_B_NK) && ragged_staged(M, K, N)) return ragged_bytes(M, K, N);
+    if ((b_layout == MAM_B_KN || b_layout == MAM_B_NK) && ragged_staged(M, K, N)) {
+        // the padded copies are as large as the operands: asked for only where the call will make them
+        const int forced = g_variant[want_indices ? 1 : 0];
+        const int variant = forced == -1 ? matrix_variant(want_indices != 0, M, N, K, b_layout, plan_dev()) : forced;
+        return variant >= 0 ? ragged_bytes(M, K, N) : 0;
+    }
     if (b_layout == MAM_B_KN && K > 0 && N > 0 && K % 4 == 0) return round256((size_t)K * (size_t)N * 4);
     return 0;
 }
@@ -762,7 +800,7 @@ int mam_fwd_drop_f32(const float* a, const float* b, int b_layout, const float* 
     const bool ragged = variant != -2 && ragged_staged(M, K, N) && K / FWD_BK < 65534 && workspace != nullptr &&
                         workspace_bytes >= ragged_bytes(M, K, N) && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0;
     if (variant == -1) {
-        variant = tma_ok || ragged ? matrix_variant(want_idx, M, N, K, *d) : -2;
+        variant = tma_ok || ragged ? matrix_variant(want_idx, M, N, K, b_layout, *d) : -2;
         // b[K,N] without scratch for its copy: served by the any-shape kernel below 4096 outputs, refused above,
         // whichever kernel the sizes would take with it
         if (tma_ok && b_layout == MAM_B_KN &&

@@ -113,10 +113,12 @@ def test_sliced_forms(shape, variant, cuda):
 
 
 @pytest.mark.parametrize("layout", [capi.KN, capi.NK])
-@pytest.mark.parametrize("shape", [(64, 257, 64), (131, 1001, 129), (1, 2047, 600), (700, 33, 515), (2100, 70, 1030)])
+@pytest.mark.parametrize("shape", [(64, 257, 64), (131, 1001, 129), (1, 2047, 600), (700, 33, 515), (2100, 70, 1030),
+                                   (5000, 133, 1030), (38100, 245, 70), (38100, 27, 70)])
 def test_ragged_k(shape, layout, cuda):
-    """K that is no multiple of 4, large enough for the padded copies: the automatic choice against the oracle, with
-    ties at the last (repeated) element."""
+    """K that is no multiple of 4, large enough for the padded copies: the automatic choice (any-shape kernel, or copies
+    and the sliced or, beyond 592 tiles, the tiled kernel and the resolver) against the oracle, with ties at the last
+    (repeated) element."""
     M, K, N = shape
     g = torch.Generator().manual_seed(M + K * 3 + N)
     a = torch.randn(M, K, generator=g)
@@ -156,6 +158,20 @@ def test_nan_and_infinite_products(shape, variant, layout, cuda):
     assert torch.equal(imax.cpu().long(), torch.from_numpy(imax_ref))
     assert torch.equal(imin.cpu().long(), torch.from_numpy(imin_ref))
     assert np.array_equal(y.cpu().numpy(), y_ref, equal_nan=True)
+
+
+@pytest.mark.parametrize("layout", [capi.KN, capi.NK])
+@pytest.mark.parametrize("variant", [0, 2, 5, 7, 8, 13, 18])
+@pytest.mark.parametrize("shape", [(300, 29, 150), (131, 1001, 129), (65, 258, 130)])
+def test_ragged_k_in_every_kernel(shape, variant, layout, cuda):
+    """Padded copies into the tiled and sliced configurations: rows of 1, 2 and 3 elements beyond a multiple of 4, ties."""
+    M, K, N = shape
+    g = torch.Generator().manual_seed(M + K * 3 + N)
+    a, w = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g)
+    a[::2], w[::2] = a[::2].round(), w[::2].round()
+    a[0, -1], w[0, -1], w[-1, -1] = 40.0, 40.0, -40.0
+    y_ref, imax_ref, imin_ref = c_oracle.forward(a.numpy(), w.numpy(), b_is_nk=True)
+    _check_forward(a.numpy(), np.ascontiguousarray(w.numpy().T), y_ref, imax_ref, imin_ref, cuda, variant, layout)
 
 
 @pytest.mark.parametrize("shape,status", [((8, 64, 100), 0), ((1, 1024, 4095), 0), ((64, 36, 64), 3), ((131, 1001, 129), 0)])

@@ -223,3 +223,19 @@ def test_overlapped_grad_sync_is_inert_without_gradients():
     sync.finish()
     assert torch.equal(p.grad, torch.full((3,), 2.0))
     sync.remove()
+
+
+def test_padded_copies_are_asked_for_only_where_they_are_made():
+    """K % 4 != 0: scratch for the padded copies of both operands where the tiled or sliced kernels take the product,
+    none where the any-shape kernel is the faster one (short K over many rows: a convolution's first layer)."""
+    L = _lib.lib()
+    for layout in (_lib.MAM_B_KN, _lib.MAM_B_NK):
+        for M, K, N in [(65536, 27, 64), (100352, 9, 32), (401408, 27, 128), (401408, 147, 64), (1000000, 9, 64), (12608, 77, 768)]:
+            assert L.mam_fwd_workspace_bytes(M, K, N, layout, 1) == 0
+        for M, K, N in [(65536, 27, 64), (100352, 9, 32), (1000000, 9, 64)]:
+            assert L.mam_fwd_workspace_bytes(M, K, N, layout, 0) == 0
+        for M, K, N in [(401408, 147, 128), (12608, 769, 3072), (777, 1001, 515)]:
+            pitch = (K + 3) // 4 * 4
+            for idx in (0, 1):
+                need = L.mam_fwd_workspace_bytes(M, K, N, layout, idx)
+                assert (M + N) * pitch * 4 <= need <= (M + N) * pitch * 4 + 512
