@@ -77,12 +77,17 @@ Fwd forward_impl(const at::Tensor& a, const at::Tensor& w, int b_layout, const c
         dense_c = dense->contiguous();
         dense_p = dense_c.data_ptr<float>();
     }
-    const size_t ws_bytes = mam_fwd_workspace_bytes(M, K, N, b_layout, want_idx);
+    size_t ws_bytes = mam_fwd_workspace_bytes(M, K, N, b_layout, want_idx);
     at::Tensor ws;
     void* ws_p = nullptr;
     if (ws_bytes) {
-        ws = at::empty({(int64_t)ws_bytes}, a.options().dtype(at::kByte));
-        ws_p = ws.data_ptr();
+        try {
+            ws = at::empty({(int64_t)ws_bytes}, a.options().dtype(at::kByte));
+            ws_p = ws.data_ptr();
+        } catch (const c10::OutOfMemoryError&) {
+            if (K % 4 == 0) throw;
+            ws_bytes = 0;   // the padded copies of a ragged K only buy speed: the any-shape kernel needs none
+        }
     }
     auto stream = at::cuda::getCurrentCUDAStream();
     TORCH_CHECK(drop_rate >= 0.0 && drop_rate < 1.0, "drop_rate must be in [0, 1)");

@@ -174,6 +174,27 @@ def test_ragged_k_in_every_kernel(shape, variant, layout, cuda):
     _check_forward(a.numpy(), np.ascontiguousarray(w.numpy().T), y_ref, imax_ref, imin_ref, cuda, variant, layout)
 
 
+def test_ragged_k_without_memory_for_the_copies(cuda):
+    """The padded copies are as large as the operands; where they do not fit any more the call still runs."""
+    from mamtorch_b200 import _lib
+
+    M, K, N = 150000, 1001, 8
+    g = torch.Generator(device=cuda).manual_seed(3)
+    x, w = torch.randn(M, K, generator=g, device=cuda), torch.randn(N, K, generator=g, device=cuda)
+    need = _lib.lib().mam_fwd_workspace_bytes(M, K, N, capi.NK, 0)
+    op = lambda: torch.ops.mamtorch_b200.linear_forward(x, w, None, None, 1.0, 0.0, False)[0]
+    y = op()
+    torch.cuda.empty_cache()
+    limit = torch.cuda.memory_reserved() + need // 2
+    assert need > x.numel() * 4
+    torch.cuda.set_per_process_memory_fraction(limit / torch.cuda.get_device_properties(0).total_memory)
+    try:
+        short = op()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.equal(short, y)
+
+
 @pytest.mark.parametrize("shape,status", [((8, 64, 100), 0), ((1, 1024, 4095), 0), ((64, 36, 64), 3), ((131, 1001, 129), 0)])
 def test_column_major_weight_without_workspace(shape, status, cuda):
     """b[K,N] and no scratch: small products and K % 4 != 0 run in the any-shape kernel, others are refused."""
