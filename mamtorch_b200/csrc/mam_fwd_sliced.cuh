@@ -31,6 +31,9 @@ struct SlicedCfg {
     static constexpr int ID_BYTES = TRACK ? 2 * SLOTS * THREADS * 2 : 0;
     static constexpr int BAR_BYTES = 2 * STAGES * 8;
     static constexpr int SMEM_BYTES = 1024 + RING_BYTES + BAR_BYTES + ID_BYTES;
+    // CTAs per SM that shared memory leaves room for, with the registers to match: the 32x64 tile runs 5 (values) and 4
+    // (indices) of them; one fewer costs a fifth (68x1780x2415 with indices 60 -> 76 us, 11773x64x4 values 11 -> 14)
+    static constexpr int MIN_CTAS = THREADS > 128 ? 1 : TRACK ? 512 / THREADS : THREADS == 128 ? 5 : 4;
     static_assert(TM % 2 == 0, "row swizzle keys assume an even TM");
     static_assert(BM <= 256 && BN <= 256, "TMA box rows");
     static_assert(PART_BYTES <= RING_BYTES, "the partial extremes reuse the operand ring");
@@ -112,11 +115,12 @@ struct SlicedParams {
     EpilogueArgs ep;
     float one;        // 1.0f kept opaque to the compiler
     int* error;
+    unsigned wait_limit;   // polls before a wait of the chunk loop gives up
 };
 
 // grid: tiles x cluster size, consecutive CTAs form the cluster of one tile; tiles n-fastest.
 template <class Cfg>
-__global__ void __launch_bounds__(Cfg::THREADS)
+__global__ void __launch_bounds__(Cfg::THREADS, Cfg::MIN_CTAS)
 mam_fwd_sliced_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW,
                       const SlicedParams prm) {
     constexpr int TM = Cfg::TM, TN = Cfg::TN, STAGES = Cfg::STAGES, THREADS = Cfg::THREADS;
@@ -155,8 +159,9 @@ mam_fwd_sliced_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         tma_load_2d(dst, &tmA, &full_bar[s], c * FWD_BK, (int)m0);
         tma_load_2d(dst + Cfg::A_BYTES, &tmW, &full_bar[s], c * FWD_BK, (int)n0);
     };
+    int issued = 0;   // copies of chunks, counted by the thread that issues them
     if (tid == 0)
-        for (int c = c_begin; c < c_end && c < c_begin + STAGES; ++c) issue(c);
+        for (int c = c_begin; c < c_end && c < c_begin + STAGES; ++c, ++issued) issue(c);
 
     const int wm = warp / Cfg::WN, wn = warp % Cfg::WN, lane_m = lane >> 3, lane_n = lane & 7;
     const int a_first = wm * 4 * TM + lane_m, w_first = wn * 8 * TN + lane_n;
@@ -178,11 +183,13 @@ mam_fwd_sliced_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         for (int s = 0; s < 2 * Cfg::SLOTS; ++s) sts16_s(id_addr + s * THREADS * 2, (unsigned)c_begin);
     }
 
+    // After a wait that gave up nothing more is waited for, released or issued (by the lane concerned; a stage is released
+    // by lanes that saw its copy land, and the issuing thread saw it released): the loop runs out on what the ring
+    // holds, and the CTA comes to the cluster barriers with its copies waited for below.
+    bool ok = true;
     for (int c = c_begin; c < c_end; ++c) {
         const int it = c - c_begin, s = it % STAGES;
-        // a wait that gives up invalidates the result and is reported; the loop goes on so that every copy
-        // issued is waited for and every CTA reaches the cluster barriers
-        if (!mbar_wait_bounded(&full_bar[s], (uint32_t)(it / STAGES) & 1u)) atomicExch(prm.error, 1);
+        ok = ok && mbar_wait_bounded(&full_bar[s], (uint32_t)(it / STAGES) & 1u, prm.wait_limit);
         const uint32_t ap = smem_base + (uint32_t)(s * Cfg::STAGE_BYTES) + a_row0;
         const uint32_t wp = smem_base + (uint32_t)(s * Cfg::STAGE_BYTES) + w_row0;
         float lmax[TRACK ? TM : 1][TRACK ? TN : 1], lmin[TRACK ? TM : 1][TRACK ? TN : 1];
@@ -218,10 +225,13 @@ mam_fwd_sliced_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 #pragma unroll 1
         for (uint32_t qoff = 16u; qoff < qend; qoff += 16u) quad(qoff, false);
         __syncwarp();
-        if (lane == 0) mbar_arrive(&empty_bar[s]);
-        if (tid == 0 && c + STAGES < c_end) {   // refill the stage once every warp has left it
-            if (!mbar_wait_bounded(&empty_bar[s], (uint32_t)(it / STAGES) & 1u)) atomicExch(prm.error, 1);
-            issue(c + STAGES);
+        if (lane == 0 && ok) mbar_arrive(&empty_bar[s]);
+        if (tid == 0 && ok && c + STAGES < c_end) {   // refill the stage once every warp has left it
+            ok = mbar_wait_bounded(&empty_bar[s], (uint32_t)(it / STAGES) & 1u, prm.wait_limit);
+            if (ok) {
+                issue(c + STAGES);
+                ++issued;
+            }
         }
         __syncwarp();
         if constexpr (TRACK) {
@@ -250,16 +260,26 @@ mam_fwd_sliced_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         }
     }
 
-    // ---- meet: extremes into the ring (every copy into it has landed and been read), then reduce over the ranks
-    __syncthreads();
+    // ---- meet: extremes into the ring, then reduce over the ranks.  Every copy into the ring has landed and been read --
+    // or a wait gave up: then the flag is set, the last copy of each stage is waited for once more (no CTA leaves with
+    // copies in flight) and the ring is left alone; what the peers read from it is memory of this CTA all the same.
+    const bool failed = __syncthreads_or(!ok);
+    if (failed && tid == 0) {
+        atomicExch(prm.error, 1);
+        for (int it = max(0, issued - STAGES); it < issued; ++it)
+            mbar_wait_bounded(&full_bar[it % STAGES], (uint32_t)(it / STAGES) & 1u);
+    }
     float* part = reinterpret_cast<float*>(smem) + tid;     // [2 * slot + side][thread]
+    if (!failed) {
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
+        for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            part[(2 * (i * TN + j) + 0) * THREADS] = vmax[i][j];
-            part[(2 * (i * TN + j) + 1) * THREADS] = vmin[i][j];
-        }
+            for (int j = 0; j < TN; ++j) {
+                part[(2 * (i * TN + j) + 0) * THREADS] = vmax[i][j];
+                part[(2 * (i * TN + j) + 1) * THREADS] = vmin[i][j];
+            }
+    }
+    __syncwarp();
     cluster_barrier();
     const uint32_t part_addr = smem_u32(part);
     for (uint32_t slot = rank; slot < (uint32_t)Cfg::SLOTS; slot += ranks) {
