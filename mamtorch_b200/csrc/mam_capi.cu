@@ -352,12 +352,13 @@ double copies_us(int64_t M, int64_t K, int64_t N) {
 
 // Predicted time (us) of a tiled forward.  With indices the resolver is included, whose rounds cost by the share of their
 // 128 columns that exist: least-squares fit to 67 products of 64 to 400000 rows, 6 to 930 k and 1 to 4019 columns, within
-// 35 % (15470x144x65, two rounds: 80, measured 76).  Values: up to four rounds by whole chunks; beyond, where K may be
+// 35 %, the resolver's rounds dearer where there are up to four of them (15470x144x65, two rounds: 87, measured 76;
+// 1216x100x789, one round: 54, measured 56).  Values: up to four rounds by whole chunks; beyond, where K may be
 // short (the any-shape kernel is only compared with then), by K: fit to 83 such products within 33 %.
 double tiled_us(int variant, bool want_idx, int64_t M, int64_t N, int64_t K, bool many, const DevInfo& d) {
     const long long bm = want_idx ? 64 : variant == 2 ? 128 : variant == 3 ? 96 : 64, ntn = (N + 127) / 128;
     const double rounds = (double)(((M + bm - 1) / bm * ntn + d.sms - 1) / d.sms), nk = (double)((K + FWD_BK - 1) / FWD_BK);
-    if (want_idx) return 5.0 + rounds * (0.096 * K + 0.69 * nk + 5.9 + 28.4 * (double)N / (128.0 * ntn));
+    if (want_idx) return 5.0 + rounds * (0.096 * K + 0.69 * nk + 5.9 + (many ? 28.4 : 35.0) * (double)N / (128.0 * ntn));
     if (!many) return bm == 128 ? 6.1 + 6.1 * rounds * nk : bm == 96 ? 3.0 + 4.9 * rounds * nk : 0.8 + rounds * (3.2 * nk + 3.4);
     return bm == 128 ? 1.0 + rounds * (0.166 * K + 0.75 * nk + 6.7)
          : bm == 96  ? 1.4 + rounds * (0.135 * K + 0.36 * nk + 3.7)
