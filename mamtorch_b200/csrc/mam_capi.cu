@@ -705,10 +705,11 @@ size_t mam_fwd_workspace_bytes(int64_t M, int64_t K, int64_t N, int b_layout, in
     return 0;
 }
 
-// Slabs of rows for mam_colsum_f32: about four CTAs per SM and at least 64 rows each.
+// Row slabs of mam_colsum_f32: as many as keep the grid within COLSUM_CTAS CTAs of each of a B200's 148 SMs, but no
+// more than one per 64 rows.  The SM count is a constant of the plan, so that the size query and the launch agree.
 static int64_t colsum_slabs(int64_t M, int64_t N) {
     const int64_t groups = (N + COLSUM_COLS - 1) / COLSUM_COLS;
-    int64_t slabs = (8 * 148 + groups - 1) / groups;
+    int64_t slabs = COLSUM_CTAS * 148 / groups;
     if (slabs > (M + 63) / 64) slabs = (M + 63) / 64;
     return slabs < 1 ? 1 : slabs;
 }

@@ -437,8 +437,7 @@ at::Tensor conv_channels_last(const at::Tensor& x) {
                  "mam_nchw_to_nhwc_f32");
     return out;
 }
-// A fresh contiguous [C,R] transpose of the matrix a[R,C] (the same batched-transpose kernel, one image of R
-// channels and C pixels); several times faster than a strided torch copy.
+// out[n] = sum over m of a[m][n] (the bias gradient)
 at::Tensor column_sum(const at::Tensor& a) {
     TORCH_CHECK(a.is_cuda() && a.scalar_type() == at::kFloat && a.dim() == 2, "a must be a float32 CUDA matrix");
     auto ac = a.contiguous();
@@ -454,6 +453,8 @@ at::Tensor column_sum(const at::Tensor& a) {
                  "mam_colsum_f32");
     return out;
 }
+// A fresh contiguous [C,R] transpose of the matrix a[R,C] (the same batched-transpose kernel, one image of R
+// channels and C pixels); several times faster than a strided torch copy.
 at::Tensor transpose2d(const at::Tensor& a) {
     TORCH_CHECK(a.is_cuda() && a.scalar_type() == at::kFloat && a.dim() == 2, "a must be a float32 CUDA matrix");
     auto ac = a.contiguous();

@@ -163,12 +163,46 @@ def test_selection_count_large(cuda):
     assert torch.equal(hmax.cpu(), rmax) and torch.equal(hmin.cpu(), rmin)
 
 
-@pytest.mark.parametrize("shape", [(1, 1), (63, 31), (64, 33), (4097, 32), (129, 4099), (70001, 17), (12608, 768)])
+@pytest.mark.parametrize("shape", [(1, 1), (63, 31), (64, 33), (4097, 32), (129, 4099), (70001, 17), (12608, 768),
+                                   (100003, 641), (70000, 1024)])
 def test_column_sum(shape, cuda):
-    """Column sums against float64 at the edges of slabs, lanes and column groups.  Each sum is a tree of at most
-    M/64 + 64 sequential fp32 additions, so its error stays below (M/64 + 64) * 2^-24 of the sum of magnitudes."""
+    """Column sums against float64 at the edges of slabs, lanes, runs and column groups.  A term passes through at most 16
+    additions of its run, one per run of its thread (512 rows of the slab each), 3 of the rows beyond the last four-row
+    step, 2 + 3 that join accumulators and lanes, and the same again over the slabs: the error stays below that many
+    2^-24 of the sum of magnitudes."""
+    from mamtorch_b200 import _lib
+
     M, N = shape
     a = torch.randn(M, N, generator=torch.Generator().manual_seed(M + N)).to(cuda)
     got = torch.ops.mamtorch_b200.column_sum(a).double()
-    bound = (M / 64 + 64) * 2.0 ** -24 * a.double().abs().sum(0)
+    slabs = _lib.lib().mam_colsum_workspace_bytes(M, N) // (4 * N)
+    depth = sum(16 + rows // 512 + 16 + 3 + 2 + 3 for rows in (-(-M // slabs), slabs))
+    bound = depth * 2.0 ** -24 * a.double().abs().sum(0)
     assert got.shape == (N,) and bool(((got - a.double().sum(0)).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("shape", [(401408, 1000), (300000, 1024), (401408, 128)])
+def test_column_sum_is_no_less_precise_than_torch(shape, cuda):
+    """Long slabs: 2-norm error against float64 at most torch's (it was 1.4 times torch's with one run per slab)."""
+    a = torch.randn(*shape, generator=torch.Generator(device=cuda).manual_seed(1), device=cuda)
+    want = sum(part.double().sum(0) for part in a.split(50000))
+    err = lambda t: float((t.double() - want).norm())
+    assert err(torch.ops.mamtorch_b200.column_sum(a)) <= 1.1 * err(a.sum(0))
+
+
+def test_bias_gradient_dispatch(cuda):
+    """At a size where the library's kernel sums the columns: the module's bias gradient, and under create_graph a
+    gradient that can be differentiated again."""
+    from mamtorch_b200.nn import FullyConnected
+
+    layer = FullyConnected(16, 64, device=cuda)
+    g = torch.Generator(device=cuda).manual_seed(2)
+    x = torch.randn(1 << 14, 16, generator=g, device=cuda)
+    gy = torch.randn(1 << 14, 64, generator=g, device=cuda).requires_grad_()
+    db, = torch.autograd.grad(layer(x), layer.bias, gy.detach())
+    assert torch.equal(db, torch.ops.mamtorch_b200.column_sum(gy.detach()))
+    want = gy.detach().double().sum(0)
+    assert float((db.double() - want).abs().max()) <= 1e-5 * float(gy.detach().abs().sum(0).max())
+    db2, = torch.autograd.grad(layer(x), layer.bias, gy, create_graph=True)
+    ggy, = torch.autograd.grad(db2.sum(), gy)
+    assert torch.equal(ggy, torch.ones_like(gy))
