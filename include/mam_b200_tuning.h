@@ -20,9 +20,7 @@ enum mam_tune_knob {
     MAM_TUNE_BWD_FORM = 3,     /* 0 by shape, 1 CTA-shared rows of dX, 2 separate dX and dW kernels,
                                   3 / 4 one row of dX per warp (a parked in shared memory / read through L1)  */
     MAM_TUNE_DENSE_SPLIT = 4,  /* TF32 product: 1 slices the tiles of the last partial wave (default), 0 not  */
-    MAM_TUNE_CONV_DIRECT_ROWS = 5, /* output rows per CTA of the one-kernel convolution backward, 0 by size   */
-    MAM_TUNE_SLICED_WAITS = 6  /* polls before a wait of the sliced forward gives up: -1 the library's limit, 0 at
-                                  once (the call then reports MAM_ERR_DEVICE_TIMEOUT and its outputs are invalid) */
+    MAM_TUNE_CONV_DIRECT_ROWS = 5 /* output rows per CTA of the one-kernel convolution backward, 0 by size    */
 };
 
 /* Sets one knob; MAM_ERR_INVALID_ARGUMENT for an unknown knob or a value outside its range. */

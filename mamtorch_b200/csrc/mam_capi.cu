@@ -238,7 +238,6 @@ const char* kSlicedNames[N_SLICED] = {"sliced_t8x128_s1", "sliced_t8x128_s2", "s
                                       "sliced_t64x128_s1", "sliced_t64x128_s2", "sliced_t64x128_s4",
                                       "sliced_t64x128_s8"};
 int g_variant[2] = {-1, -1};  // [with_indices]
-unsigned g_sliced_waits = 1u << 22;   // polls before a wait of the sliced kernel gives up
 int g_resolve_simple = 0;      // 1: use the thread-per-output resolver (cross-check)
 
 // Scratch for mam_fwd_kn_static_f32: lives in the library image, one copy per device.
@@ -450,7 +449,7 @@ int run_tiled(const float* a, const float* w, float* y, int32_t* argmax, int32_t
     int* flag = nullptr;
     MAM_CUDA(cudaGetSymbolAddress(reinterpret_cast<void**>(&flag), g_wait_gave_up));
     if (!cv && variant >= N_TILED) {
-        const SlicedParams sp{a, w, y, argmax, argmin, M, K, N, ep, 1.0f, flag, g_sliced_waits};
+        const SlicedParams sp{a, w, y, argmax, argmin, M, K, N, ep, 1.0f, flag};
         return want_idx ? run_sliced<true>(sp, variant - N_TILED, d, cs) : run_sliced<false>(sp, variant - N_TILED, d, cs);
     }
     FwdParams prm{y, argmax, argmin, M, K, N, ep, 1.0f, flag, Im2colRows{}, 0};
@@ -676,10 +675,6 @@ int mam_tune_set(int knob, int value) {
         case MAM_TUNE_CONV_DIRECT_ROWS:
             if (value < 0 || value > 64) return MAM_ERR_INVALID_ARGUMENT;
             g_conv_direct_rows = value;
-            return MAM_OK;
-        case MAM_TUNE_SLICED_WAITS:
-            if (value < -1) return MAM_ERR_INVALID_ARGUMENT;
-            g_sliced_waits = value == -1 ? 1u << 22 : (unsigned)value;
             return MAM_OK;
         default:
             return MAM_ERR_INVALID_ARGUMENT;

@@ -115,7 +115,6 @@ struct SlicedParams {
     EpilogueArgs ep;
     float one;        // 1.0f kept opaque to the compiler
     int* error;
-    unsigned wait_limit;   // polls before a wait of the chunk loop gives up
 };
 
 // grid: tiles x cluster size, consecutive CTAs form the cluster of one tile; tiles n-fastest.
@@ -189,7 +188,7 @@ mam_fwd_sliced_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     bool ok = true;
     for (int c = c_begin; c < c_end; ++c) {
         const int it = c - c_begin, s = it % STAGES;
-        ok = ok && mbar_wait_bounded(&full_bar[s], (uint32_t)(it / STAGES) & 1u, prm.wait_limit);
+        ok = ok && mbar_wait_bounded(&full_bar[s], (uint32_t)(it / STAGES) & 1u);
         const uint32_t ap = smem_base + (uint32_t)(s * Cfg::STAGE_BYTES) + a_row0;
         const uint32_t wp = smem_base + (uint32_t)(s * Cfg::STAGE_BYTES) + w_row0;
         float lmax[TRACK ? TM : 1][TRACK ? TN : 1], lmin[TRACK ? TM : 1][TRACK ? TN : 1];
@@ -227,7 +226,7 @@ mam_fwd_sliced_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         __syncwarp();
         if (lane == 0 && ok) mbar_arrive(&empty_bar[s]);
         if (tid == 0 && ok && c + STAGES < c_end) {   // refill the stage once every warp has left it
-            ok = mbar_wait_bounded(&empty_bar[s], (uint32_t)(it / STAGES) & 1u, prm.wait_limit);
+            ok = mbar_wait_bounded(&empty_bar[s], (uint32_t)(it / STAGES) & 1u);
             if (ok) {
                 issue(c + STAGES);
                 ++issued;

@@ -215,30 +215,6 @@ def test_column_major_weight_without_workspace(shape, status, cuda):
         assert torch.equal(imin.cpu().long(), torch.from_numpy(imin_ref))
 
 
-@pytest.mark.parametrize("want_idx", [True, False])
-@pytest.mark.parametrize("variant", [8, 10, 15, 19])
-def test_sliced_waits_that_run_out_are_reported(variant, want_idx, cuda):
-    """With a limit of no polls at all the kernel ends by itself with the flag set, and the next call is right."""
-    from mamtorch_b200 import _lib
-
-    g = torch.Generator().manual_seed(variant)
-    a, w = torch.randn(40, 2084, generator=g), torch.randn(70, 2084, generator=g)
-    y_ref, imax_ref, _ = c_oracle.forward(a.numpy(), w.numpy(), b_is_nk=True)
-    L = _lib.lib()
-    capi.set_variant(want_idx, variant)
-    try:
-        _lib.check(L.mam_tune_set(6, 0), "wait limit")
-        capi.forward(a.to(cuda), w.to(cuda), capi.NK, want_idx=want_idx)
-        assert L.mam_check_device_flag() == 5
-        _lib.check(L.mam_tune_set(6, -1), "wait limit")
-        y, imax, _ = capi.forward(a.to(cuda), w.to(cuda), capi.NK, want_idx=want_idx)
-    finally:
-        capi.set_variant(want_idx, -1)
-        L.mam_tune_set(6, -1)
-    assert capi.device_flag_ok() and torch.equal(y.cpu(), torch.from_numpy(y_ref))
-    assert not want_idx or torch.equal(imax.cpu().long(), torch.from_numpy(imax_ref))
-
-
 RESOLVER_SHAPES = [(300, 260, 200), (65, 4, 63), (129, 2080, 131), (257, 96, 129), (520, 2500, 140), (64, 2048, 64),
                    (1, 64, 1), (200, 416, 136)]
 
