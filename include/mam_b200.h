@@ -69,7 +69,12 @@ int mam_poll_device_flag(void* stream);
 int mam_timer_arm(void** starts, void** stops, int capacity, int kernel_id);
 int mam_timer_disarm(void);
 
-/* Workspace needed by mam_fwd_f32 for these extents (0 is possible). */
+/* Scratch mam_fwd_f32 wants for these extents and outputs (0 is possible), 256-byte aligned.
+ *   K % 4 == 0, MAM_B_KN: the transposed copy of b.  Required from 4096 outputs on (MAM_ERR_WORKSPACE without it, where
+ *     both operands are 16-byte aligned); below, the call runs without.
+ *   K % 4 != 0, either layout: padded copies of both operands, asked for only where they make the call faster (products
+ *     from M*K*N = 2^20 on, not for short K over many rows).  Optional: without it the any-shape kernel runs.
+ *   K % 4 == 0, MAM_B_NK: none. */
 size_t mam_fwd_workspace_bytes(int64_t M, int64_t K, int64_t N, int b_layout, int want_indices);
 
 /* MAM forward.
