@@ -250,8 +250,8 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 size_t round256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // K not a multiple of 4: both operands are copied once with padded rows (mam_stage_ragged_kernel) so that TMA can
-// read them, where the product is large enough for the copy's launch: at 64x257x64 (2^20 units) the any-shape kernel
-// takes about 70 us and the copy with the sliced kernel about 15.
+// read them, where the product is large enough for the copy's launch (at 64x257x64, 2^20 units, the any-shape kernel
+// takes about 70 us and the copy with the sliced kernel about 15) and matrix_variant finds the copies worth it.
 bool ragged_staged(int64_t M, int64_t K, int64_t N) {
     return M > 0 && N > 0 && K > 4 && K % 4 != 0 && (double)M * (double)K * (double)N >= 1048576.0;
 }

@@ -32,7 +32,7 @@ struct SlicedCfg {
     static constexpr int BAR_BYTES = 2 * STAGES * 8;
     static constexpr int SMEM_BYTES = 1024 + RING_BYTES + BAR_BYTES + ID_BYTES;
     // CTAs per SM that shared memory leaves room for, with the registers to match: the 32x64 tile runs 5 (values) and 4
-    // (indices) of them; one fewer costs a fifth (68x1780x2415 with indices 60 -> 76 us, 11773x64x4 values 11 -> 14)
+    // (indices) of them; one fewer costs a fifth (68x1780x2415 with indices 60 -> 76 us, 11773x62x4 values 13.5 -> 16.5)
     static constexpr int MIN_CTAS = THREADS > 128 ? 1 : TRACK ? 512 / THREADS : THREADS == 128 ? 5 : 4;
     static_assert(TM % 2 == 0, "row swizzle keys assume an even TM");
     static_assert(BM <= 256 && BN <= 256, "TMA box rows");

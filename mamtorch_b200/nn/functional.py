@@ -198,7 +198,7 @@ def poll_device_flag() -> None:
 def bias_grad(gy: Tensor) -> Tensor:
     """Column sums of the upstream gradient [M,N].  The library's kernel, where it was measured to be the faster one and no
     less precise: narrow matrices of many rows (back to back [401408,128] 41 us against 188 for `sum(0)`, [12608,768] 14
-    against 24, errors against float64 1.2e-7 / 4.2e-7 and 1.1e-7 / 1.4e-7; over 90 shapes of 2^20 to 4 * 10^8 elements
+    against 24, errors against float64 1.2e-7 / 4.2e-7 and 1.1e-7 / 1.4e-7; over 80 shapes of 2^20 to 4 * 10^8 elements
     device time 0.18 to 0.90 of torch's).  Torch's sum stays for wide ones ([12608,3072] 33 against 39, little to gain),
     below 32 columns (lanes idle) or 2^20 elements (two launches: [4096,256] 14.4 against 14.2), and under
     `create_graph`, where the sum has to stay differentiable."""
